@@ -475,21 +475,11 @@ gemm_tc_wide_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
     }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
-  if (warp == 1) {
-    asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_holder)), "r"(512u) : "memory");
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
-  }
-  tc_fence_before();
   __syncthreads();
-  cluster_sync();
-  tc_fence_after();
-  const uint32_t tmem = tmem_holder;
+  cluster_sync();            // both CTAs run and their barriers can be used from the other one
   volatile int* ab = &abort_flag;
 
-  // Dependents start only now that every block has its tensor memory: one of them that took tensor memory first and waited
-  // for this kernel would keep it waiting.
   if (map_pending) pdl_wait();
-  pdl_launch();
   const int tiles_n = grouped ? *p.n_tiles : (p.rows + p.row_step - 1) / p.row_step;
   const int n_items = tiles_m * tiles_n * p.splits;
 
@@ -518,38 +508,62 @@ gemm_tc_wide_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
     return true;
   };
 
+  auto load_w = [&](const Item& w, int s, int i) {
+    tma_load_2d_pair(tiles + s * STAGE_BYTES, &map_w, (w.kb0 + i) * BK, w.w_row, full0 + 8 * s);
+  };
+  auto load_x = [&](const Item& w, int s, int i) {
+    const int half = w.mma_n >> 1;
+    for (int b = 0; b * p.x_box < half; ++b)
+      tma_load_2d_pair(tiles + s * STAGE_BYTES + A_BYTES + b * p.x_box * BK * 2, &map_x, (w.kb0 + i) * BK,
+                       w.row0 + rank * half + b * p.x_box, full0 + 8 * s);
+  };
+  auto expect = [&](const Item& w, int s) {          // what both CTAs bring
+    if (rank == 0) mbar_expect_tx(full0 + 8 * s, 2 * (A_BYTES + ((w.mma_n >> 1) + p.x_box - 1) / p.x_box * p.x_box * BK * 2));
+  };
+  // the weights of the first ring do not depend on the kernel before this one
+  int ahead = 0;
+  if (warp == 0 && lane == 0) {
+    Item w;
+    if (item_at(pair, w)) {
+      ahead = w.nkb < WIDE_STAGES ? w.nkb : WIDE_STAGES;
+      for (int i = 0; i < ahead; ++i) {
+        expect(w, i);
+        load_w(w, i, i);
+      }
+    }
+  }
+  // Tensor memory is taken by a pair that has met, when every earlier kernel has ended, and dependents start only when every
+  // pair has its own: no wait for tensor memory (it has no limit) can then stand against another kernel's.  Taken at the top,
+  // by each CTA before it knew of the other and beside earlier kernels' blocks, prompts of 470 rows and more through four
+  // layers of width 2,048 did not end.
+  pdl_wait();
+  __syncwarp();
+  if (warp == 1) {
+    asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_holder)), "r"(512u) : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+  }
+  tc_fence_before();
+  __syncthreads();
+  cluster_sync();
+  tc_fence_after();
+  const uint32_t tmem = tmem_holder;
+  pdl_launch();
+
   if (warp == 0 && lane == 0) {
     // ---------------------------------------------------------------- TMA producer of this CTA's halves
     int kc = 0;
-    bool first = true, ok = true;
+    bool ok = true;
     Item w;
     for (int it = pair; ok && item_at(it, w); it += pairs) {
-      const int half = w.mma_n >> 1, boxes = (half + p.x_box - 1) / p.x_box;
-      const uint32_t box_bytes = p.x_box * BK * 2, bytes = 2 * (A_BYTES + boxes * box_bytes);
-      auto x_boxes = [&](int s, int kx) {
-        for (int b = 0; b < boxes; ++b)
-          tma_load_2d_pair(tiles + s * STAGE_BYTES + A_BYTES + b * box_bytes, &map_x, kx, w.row0 + rank * half + b * p.x_box, full0 + 8 * s);
-      };
       int i = 0;
-      if (first) {
-        // the weights of the first ring do not depend on the kernel before this one
-        const int head = w.nkb < WIDE_STAGES ? w.nkb : WIDE_STAGES;
-        for (; i < head; ++i) {
-          if (rank == 0) mbar_expect_tx(full0 + 8 * i, bytes);
-          tma_load_2d_pair(tiles + i * STAGE_BYTES, &map_w, (w.kb0 + i) * BK, w.w_row, full0 + 8 * i);
-        }
-        pdl_wait();
-        for (int j = 0; j < head; ++j) x_boxes(j, (w.kb0 + j) * BK);
-        kc = head;
-        first = false;
-      }
+      for (; i < ahead; ++i, ++kc) load_x(w, i, i);
+      ahead = 0;
       for (; i < w.nkb; ++i, ++kc) {
         const int s = kc % WIDE_STAGES;
         if (!mbar_wait(empty0 + 8 * s, ((kc / WIDE_STAGES) & 1) ^ 1, ab, p.wait_cycles)) { ok = false; break; }
-        if (rank == 0) mbar_expect_tx(full0 + 8 * s, bytes);
-        const int kx = (w.kb0 + i) * BK;
-        tma_load_2d_pair(tiles + s * STAGE_BYTES, &map_w, kx, w.w_row, full0 + 8 * s);
-        x_boxes(s, kx);
+        expect(w, s);
+        load_w(w, s, i);
+        load_x(w, s, i);
       }
     }
   } else if (warp == 1 && lane == 0 && rank == 0) {
@@ -581,14 +595,12 @@ gemm_tc_wide_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
     // ---------------------------------------------------------------- epilogue of this CTA's features
     const int q = warp & 3;
     const bool raw = p.splits > 1 || p.defer;
-    bool waited = false;
     int j = 0;
     Item w;
     for (int it = pair; item_at(it, w); it += pairs, ++j) {
       const int buf = j & 1;
       if (!mbar_wait(acc_full0 + 8 * buf, (j >> 1) & 1, ab, p.wait_cycles)) break;
       tc_fence_after();
-      if (!waited) { pdl_wait(); waited = true; }   // before reading or writing what earlier kernels touch
       const int f = GATED ? w.f0 + q * GATE_BLOCK + (lane & 15) : w.f0 + q * 32 + lane;
       const bool f_ok = f < p.N;
       const float bias = (!GATED && p.bias && f_ok && !raw) ? p.bias[f] : 0.f;

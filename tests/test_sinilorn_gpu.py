@@ -590,6 +590,39 @@ def test_a_cut_changes_float32_logits_by_rounding_only(setup):
     assert float(rel_err(got, a[0].double()).max()) < 3e-5
 
 
+# a recurrent layer and a latent one of a served width: products of hundreds of rows that fill the device several times over
+SERVED = {
+    "architecture": "Sinilorn", "vocab": 96, "width": 2048, "streams": 4, "norm": {"eps": 1e-5}, "logit_scale": 1.0,
+    "layers": [
+        tiny._layer("rglru", tiny._unit(2048, 8, 4), tiny._dense(8192)),
+        tiny._layer("latent_attention", tiny._latent(16, 128, 64, 128, 1536, 512, size=256, base=500000.0), tiny._moe(1408, 7.0, 12, 3, 4)),
+    ],
+}
+
+
+def test_prompts_of_served_sizes(ops, tmp_path):
+    """Whole prompts, and prompts whose last tokens are decoded, through layers of served sizes, every bounded wait cut to
+    some 30 ms.  Bound: as for the tiny configurations in bfloat16."""
+    cfg = SERVED
+    folder, w = tiny.write_model(tmp_path / "m", cfg, seed=5)
+    reqs = traces.make_requests(cfg["vocab"], (150, 470, 900), seed=5)
+    keep = {rid: set(range(0, len(t), 7)) | set(range(len(t) - 6, len(t))) for rid, t in reqs.items()}
+    ops.set_wait_cycles(50_000_000)
+    try:
+        steps = traces.whole(reqs, keep)
+        out, recs, _ = replay(folder, steps, "bfloat16", record={})
+        cut = traces.tail_decoded(reqs, tail=5, keep=keep)
+        decoded, _, _ = replay(folder, cut, "bfloat16")
+    finally:
+        ops.set_wait_cycles(0)
+    base = {rid: P.forward(cfg, w, t, forced=[None, recs[i]["experts"][0].cpu()])[0] for i, (rid, t) in enumerate(reqs.items())}
+    for got, exp in ((out, traces.expected_rows(steps, base)), (decoded, traces.expected_rows(cut, base))):
+        assert set(got) == set(exp)
+        errs = torch.cat([rel_err(got[k], torch.stack(rows)) for k, rows in exp.items()])
+        bad = int((errs > 8e-2).sum())
+        assert bad <= 0.1 * len(errs), f"{bad} of {len(errs)} rows, worst {float(errs.max()):.3g}"
+
+
 @pytest.mark.parametrize("seed", [11, 12, 13, 14, 15, 16, 17, 18, 19, 20])
 def test_configurations_drawn_at_random(seed, tmp_path):
     cfg = tiny.random_config(seed)
