@@ -297,9 +297,11 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
     // reference of the exponentials, sum of P: a sink is what both start from
     const float sink = p.sinks ? p.sinks[head] * 1.4426950408889634f : -INFINITY;
     float ref = fmaxf(sink, -1e30f), l = sink > -1e30f ? 1.f : 0.f;
+    // every lane of a warp goes on or none does: tensor memory is read and written by whole warps
+    auto wait = [&](uint32_t bar, uint32_t parity) { return __all_sync(0xffffffffu, mbar_wait(bar, parity, ab, p.wait_cycles)) != 0; };
     bool ok = true;
     for (int i = 0; i < n_kv_tiles && ok; ++i) {
-      ok = mbar_wait(bar_s0 + 8 * (i & 1), (i >> 1) & 1, ab, p.wait_cycles);
+      ok = wait(bar_s0 + 8 * (i & 1), (i >> 1) & 1);
       if (!ok) break;
       tc_fence_after();
       const int kv0 = (tile_lo + i) * BKV;
@@ -332,7 +334,7 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
         ref = mx;
         l *= alpha;
         if (i > 0) {
-          ok = mbar_wait(bar_o, (i - 1) & 1, ab, p.wait_cycles);
+          ok = wait(bar_o, (i - 1) & 1);
           if (!ok) break;
           o_seen = true;
           tc_fence_after();
@@ -367,7 +369,7 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
       tmem_st32(tmem_s + (i & 1) * BKV + lane_addr, packed);
       tmem_st_wait();
       if (!o_seen) {
-        ok = mbar_wait(bar_o, (i - 1) & 1, ab, p.wait_cycles);
+        ok = wait(bar_o, (i - 1) & 1);
         if (!ok) break;
       }
       l += (s4[0] + s4[1]) + (s4[2] + s4[3]);
@@ -376,7 +378,7 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
       tc_fence_before();
       mbar_arrive(bar_p);
     }
-    if (ok) ok = mbar_wait(bar_o, (n_kv_tiles - 1) & 1, ab, p.wait_cycles);
+    if (ok) ok = wait(bar_o, (n_kv_tiles - 1) & 1);
     if (ok) {
       tc_fence_after();
       pdl_wait();             // every thread that writes waits for the earlier kernels itself (long over by now)

@@ -298,7 +298,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
       const Item w = item_at(j);
       if (!w.valid) break;
       const int buf = j & 1;
-      if (!mbar_wait(acc_full0 + 8 * buf, (j >> 1) & 1, ab, p.wait_cycles)) break;
+      // every lane goes on or none does: what follows is the whole warp's
+      if (!__all_sync(0xffffffffu, mbar_wait(acc_full0 + 8 * buf, (j >> 1) & 1, ab, p.wait_cycles))) break;
       tc_fence_after();
       if (!waited) { pdl_wait(); waited = true; }   // before reading or writing what earlier kernels touch
       // output feature of this thread: its lane of the accumulator, or, gated, one of the warp's 16
@@ -431,6 +432,15 @@ __device__ __forceinline__ void umma_bf16_pair(uint32_t d_tmem, uint64_t a_desc,
       "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}"
       ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate) : "memory");
 }
+// the place of another CTA of the cluster that this CTA's place corresponds to
+__device__ __forceinline__ uint32_t place_in(uint32_t addr, uint32_t rank) {
+  uint32_t r;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
+  return r;
+}
+__device__ __forceinline__ void store_in_cluster(uint32_t addr, int v) {
+  asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(addr), "r"(v) : "memory");
+}
 __device__ __forceinline__ void umma_commit_pair(uint32_t bar) {      // arrives at this barrier of both CTAs
   asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;"
                ::"r"(bar), "h"((uint16_t)3) : "memory");
@@ -449,7 +459,7 @@ gemm_tc_wide_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
   extern __shared__ uint8_t smem_raw[];
   __shared__ __align__(8) uint64_t bars[2 * WIDE_STAGES + 4];   // full, empty, acc_full[2], acc_empty[2]
   __shared__ uint32_t tmem_holder;
-  __shared__ int abort_flag;
+  __shared__ int abort_flag, given_up;
 
   const bool grouped = p.tile_expert != nullptr;
   const bool map_pending = grouped && !p.plan_ready;
@@ -463,8 +473,10 @@ gemm_tc_wide_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int rank = (int)cluster_rank(), pair = blockIdx.x >> 1, pairs = gridDim.x >> 1;
 
+  // An earlier block gave up: do not queue up behind it.  The pair acts on what its leader saw.
+  const int seen = threadIdx.x == 0 && rank == 0 ? *(volatile int*)p.error_flag : 0;
   if (threadIdx.x == 0) {
-    abort_flag = 0;
+    abort_flag = given_up = 0;
     for (int s = 0; s < WIDE_STAGES; ++s) {
       mbar_init(full0 + 8 * s, 1);
       mbar_init(empty0 + 8 * s, 1);
@@ -477,7 +489,17 @@ gemm_tc_wide_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
   }
   __syncthreads();
   cluster_sync();            // both CTAs run and their barriers can be used from the other one
-  volatile int* ab = &abort_flag;
+  if (seen) {
+    given_up = 1;
+    store_in_cluster(place_in(smem_u32(&given_up), 1), 1);
+  }
+  // every bounded wait of the kernel; one that runs out ends those of both CTAs
+  const uint32_t peer_abort = place_in(smem_u32(&abort_flag), rank ^ 1);
+  auto wait = [&](uint32_t bar, uint32_t parity) -> bool {
+    if (mbar_wait(bar, parity, &abort_flag, p.wait_cycles)) return true;
+    store_in_cluster(peer_abort, 1);
+    return false;
+  };
 
   if (map_pending) pdl_wait();
   const int tiles_n = grouped ? *p.n_tiles : (p.rows + p.row_step - 1) / p.row_step;
@@ -549,7 +571,9 @@ gemm_tc_wide_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
   const uint32_t tmem = tmem_holder;
   pdl_launch();
 
-  if (warp == 0 && lane == 0) {
+  if (given_up) {
+    // nothing to do but to leave
+  } else if (warp == 0 && lane == 0) {
     // ---------------------------------------------------------------- TMA producer of this CTA's halves
     int kc = 0;
     bool ok = true;
@@ -560,7 +584,7 @@ gemm_tc_wide_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
       ahead = 0;
       for (; i < w.nkb; ++i, ++kc) {
         const int s = kc % WIDE_STAGES;
-        if (!mbar_wait(empty0 + 8 * s, ((kc / WIDE_STAGES) & 1) ^ 1, ab, p.wait_cycles)) { ok = false; break; }
+        if (!wait(empty0 + 8 * s, ((kc / WIDE_STAGES) & 1) ^ 1)) { ok = false; break; }
         expect(w, s);
         load_w(w, s, i);
         load_x(w, s, i);
@@ -573,14 +597,14 @@ gemm_tc_wide_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
     Item w;
     for (int it = pair; ok && item_at(it, w); it += pairs, ++j) {
       const int buf = j & 1;
-      ok = mbar_wait(acc_empty0 + 8 * buf, ((j >> 1) & 1) ^ 1, ab, p.wait_cycles);     // both epilogues have drained this set
+      ok = wait(acc_empty0 + 8 * buf, ((j >> 1) & 1) ^ 1);     // both epilogues have drained this set
       if (!ok) break;
       tc_fence_after();
       const uint32_t acc_addr = tmem + buf * WIDE_ROWS;
       const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(w.mma_n >> 3) << 17) | ((uint32_t)(2 * BM >> 4) << 24);
       for (int i = 0; i < w.nkb; ++i, ++kc) {
         const int s = kc % WIDE_STAGES;
-        ok = mbar_wait(full0 + 8 * s, (kc / WIDE_STAGES) & 1, ab, p.wait_cycles);
+        ok = wait(full0 + 8 * s, (kc / WIDE_STAGES) & 1);
         if (!ok) break;
         tc_fence_after();
         const uint32_t a = tiles + s * STAGE_BYTES, b = a + A_BYTES;
@@ -599,7 +623,8 @@ gemm_tc_wide_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
     Item w;
     for (int it = pair; item_at(it, w); it += pairs, ++j) {
       const int buf = j & 1;
-      if (!mbar_wait(acc_full0 + 8 * buf, (j >> 1) & 1, ab, p.wait_cycles)) break;
+      // every lane goes on or none does: what follows is the whole warp's
+      if (!__all_sync(0xffffffffu, wait(acc_full0 + 8 * buf, (j >> 1) & 1))) break;
       tc_fence_after();
       const int f = GATED ? w.f0 + q * GATE_BLOCK + (lane & 15) : w.f0 + q * 32 + lane;
       const bool f_ok = f < p.N;
@@ -652,8 +677,7 @@ gemm_tc_wide_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
   }
   // ---- teardown: the pair meets, then its tensor memory is freed
   tc_fence_before();
-  __syncthreads();
-  if (abort_flag) {
+  if (__syncthreads_or(abort_flag || given_up)) {      // the other CTA may still raise the flag: one answer for all threads
     if (threadIdx.x == 0) {
       atomicExch(p.error_flag, 1);
       const long long t0 = clock64();     // let copies in flight land before the block ends

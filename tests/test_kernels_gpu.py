@@ -194,6 +194,36 @@ def test_products_of_many_rows_on_pairs_of_multiprocessors(ops, M, N, K):
     assert int(ops.tc_error.item()) == 0
 
 
+@pytest.mark.parametrize("M,gated,E", [(40, False, 0), (300, False, 0), (300, True, 0), (300, True, 2), (300, False, 2)])
+def test_products_do_not_queue_up_behind_one_that_gave_up(ops, M, gated, E):
+    """With the error flag set a product returns and writes nothing; one whose own waits run out sets it; afterwards it works."""
+    g = torch.Generator().manual_seed(M + E)
+    x, w = torch.randn(M, 256, generator=g).bfloat16().to(DEV), torch.randn(max(E, 1), 2048, 256, generator=g).bfloat16().to(DEV)
+    if gated:
+        w = torch.stack([ops.pair_gate_up(a[:1024], a[1024:]) for a in w])
+    plan = None
+    if E:
+        plan, x = ops.moe_dispatch(torch.arange(M, device=DEV, dtype=torch.int32)[:, None] % E, E, 256, x)
+    out = torch.full((M, 1024 if gated else 2048), 7.0, device=DEV)
+    product = lambda: ops._gemm(x, w if E else w[0], gated, out, None, False, "silu", plan)
+    try:
+        ops.tc_error.fill_(1)
+        product()
+        assert (out == 7.0).all()
+        ops.tc_error.zero_()
+        ops.set_wait_cycles(1)
+        for _ in range(20):          # more than one of them may come through: a wait is looked at only so often
+            product()
+        torch.cuda.synchronize()
+    finally:
+        ops.set_wait_cycles(0)
+        ops.tc_error.zero_()
+    product()
+    first = out.clone()
+    product()
+    assert torch.equal(out, first) and not (out == 7.0).any() and int(ops.tc_error.item()) == 0
+
+
 @pytest.mark.parametrize("act", ["gelu", "relu2"])
 @pytest.mark.parametrize("T,N,K,E,top", [(130, 200, 64, 0, 0), (700, 264, 128, 3, 2), (90, 136, 72, 1, 1), (400, 48, 64, 5, 3)])
 def test_products_with_an_activation(ops, act, T, N, K, E, top):
