@@ -418,11 +418,11 @@ __device__ __forceinline__ uint32_t cluster_rank() {
 __device__ __forceinline__ void cluster_sync() {
   asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
-// the pair's leader holds the barrier: its address with the bit of the CTA's rank cleared
+// bar: the leader's barrier, as place_in gives it
 __device__ __forceinline__ void tma_load_2d_pair(uint32_t dst, const CUtensorMap* map, int x, int y, uint32_t bar) {
   asm volatile(
       "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
-      ::"r"(dst), "l"(map), "r"(x), "r"(y), "r"(bar & 0xFEFFFFFFu) : "memory");
+      ::"r"(dst), "l"(map), "r"(x), "r"(y), "r"(bar) : "memory");
 }
 __device__ __forceinline__ void umma_bf16_pair(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc,
                                                uint32_t accumulate) {
@@ -445,11 +445,8 @@ __device__ __forceinline__ void umma_commit_pair(uint32_t bar) {      // arrives
   asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;"
                ::"r"(bar), "h"((uint16_t)3) : "memory");
 }
-__device__ __forceinline__ void arrive_at_leader(uint32_t bar) {
-  asm volatile(
-      "{\n\t.reg .b32 r;\n\t"
-      "mapa.shared::cluster.u32 r, %0, 0;\n\t"
-      "mbarrier.arrive.release.cluster.shared::cluster.b64 _, [r];\n\t}" ::"r"(bar) : "memory");
+__device__ __forceinline__ void arrive_in_cluster(uint32_t bar) {
+  asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
 }
 
 template <bool GATED, bool RELU2>
@@ -530,14 +527,15 @@ gemm_tc_wide_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
     return true;
   };
 
+  const uint32_t leader_full = place_in(full0, 0), leader_acc_empty = place_in(acc_empty0, 0);
   auto load_w = [&](const Item& w, int s, int i) {
-    tma_load_2d_pair(tiles + s * STAGE_BYTES, &map_w, (w.kb0 + i) * BK, w.w_row, full0 + 8 * s);
+    tma_load_2d_pair(tiles + s * STAGE_BYTES, &map_w, (w.kb0 + i) * BK, w.w_row, leader_full + 8 * s);
   };
   auto load_x = [&](const Item& w, int s, int i) {
     const int half = w.mma_n >> 1;
     for (int b = 0; b * p.x_box < half; ++b)
       tma_load_2d_pair(tiles + s * STAGE_BYTES + A_BYTES + b * p.x_box * BK * 2, &map_x, (w.kb0 + i) * BK,
-                       w.row0 + rank * half + b * p.x_box, full0 + 8 * s);
+                       w.row0 + rank * half + b * p.x_box, leader_full + 8 * s);
   };
   auto expect = [&](const Item& w, int s) {          // what both CTAs bring
     if (rank == 0) mbar_expect_tx(full0 + 8 * s, 2 * (A_BYTES + ((w.mma_n >> 1) + p.x_box - 1) / p.x_box * p.x_box * BK * 2));
@@ -672,7 +670,7 @@ gemm_tc_wide_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
       }
       tc_fence_before();
       __syncwarp();
-      if (lane == 0) arrive_at_leader(acc_empty0 + 8 * buf);
+      if (lane == 0) arrive_in_cluster(leader_acc_empty + 8 * buf);
     }
   }
   // ---- teardown: the pair meets, then its tensor memory is freed
