@@ -190,6 +190,12 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
     mbar_init(bar_o, 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
+  // Tensor memory (the wait for it has no limit) is taken when every earlier kernel has ended, as in products of many rows:
+  // two blocks that took theirs early held all of a multiprocessor's, and a product before them could wait for its own while
+  // they waited for it.  Products of few rows behind this kernel may hold some by now, but no more than half beside a block
+  // of this one (shared memory has no room for more of theirs), so its blocks can always go on one by one.
+  pdl_wait();
+  __syncwarp();
   if (warp == 1) tmem_alloc(smem_u32(&tmem_holder), tmem_cols);
   tc_fence_before();
   __syncthreads();
@@ -200,9 +206,6 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
 
   if (warp == 0 && lane == 0) {
     // ---------------------------------------------------------------- loads
-    // The barriers and the tensor memory above need nothing from earlier kernels; the queries and the newest
-    // keys and values come from the kernel before this one.
-    pdl_wait();
     mbar_expect_tx(bar_q, chunks * BQ * 128);
     for (int c = 0; c < own_chunks; ++c) tma_load_2d(q_smem + c * BQ * 128, &map_q, head * p.q_step + c * 64, row0, bar_q);
     for (int c = own_chunks; c < chunks; ++c)
@@ -381,7 +384,6 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
     if (ok) ok = wait(bar_o, (n_kv_tiles - 1) & 1);
     if (ok) {
       tc_fence_after();
-      pdl_wait();             // every thread that writes waits for the earlier kernels itself (long over by now)
       const float inv = l > 0.f ? 1.0f / l : 0.f;
       __nv_bfloat16* dst = p.out + ((size_t)(row0 + r) * p.nq + head) * p.vd;
       for (int d0 = 0; d0 < p.vd; d0 += 16) {           // the loads are warp-wide: rows beyond the tile join in
