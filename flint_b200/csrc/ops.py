@@ -1067,8 +1067,9 @@ class CudaOps:
         if (tiling is not None and tiling.n_tiles > 0 and rows is None and splits is None and tiling.tile_rows > 64
                 and self.sink_attention_tiles_ok(q.dtype, cache.k.dtype, hd, vd)):
             # plain masks in tiles of up to 128 rows: the tcgen05 kernel (3,500 tokens, 32 heads of 128 in runs of 4,096: 810 us
-            # on mma.sync).  What it does not take goes to the kernel below in halves of the tiles.
-            if not keep_first and not pool and sigmoid is None and P % 8 == 0 and (64 % P == 0 or P % 64 == 0):
+            # on mma.sync).  What it does not take goes to the kernel below in halves of the tiles, cut here at the price of a
+            # wait for the device: a model's layers ask for tiles of 64 rows where they know it beforehand.
+            if not keep_first and not pool and sigmoid is None and self.prefill_pages_ok(P):
                 self._label = kind
                 self.attention_prefill_tc(q, cache, tiling.tiles, tiling.n_tiles, out, nq, nkv, hd, window, scale, vd, chunk, sinks)
                 if not tiling.n_other_rows:
@@ -1138,6 +1139,11 @@ class CudaOps:
                   c_int(_code(cache.k.dtype)), _ptr(cache.block_table), c_int(cache.block_table.shape[1]), c_int(P),
                   _ptr(step.pos), _ptr(step.slot), c_int(step.n_tokens), c_int(nkv), c_int(hd), c_int(vd), c_int(pool),
                   c_int(E), _ptr(step.status))
+
+    @staticmethod
+    def prefill_pages_ok(page_size):
+        """Whether the tcgen05 attention of prompts takes pages of this size."""
+        return page_size % 8 == 0 and (64 % page_size == 0 or page_size % 64 == 0)
 
     @staticmethod
     def sink_attention_tiles_ok(q_dtype, cache_dtype, hd, vd):

@@ -146,7 +146,7 @@ class Model:
         self.max_context = int(max_context or spec.max_positions)
         if self.max_context > spec.max_positions:
             raise ConfigError(f"max_context {self.max_context} exceeds the model's {spec.max_positions} positions")
-        self.ctx = BuildContext(ops=ops, device=self.device, compute=dtype, max_context=self.max_context)
+        self.ctx = BuildContext(ops=ops, device=self.device, compute=dtype, max_context=self.max_context, page_size=page_size)
         self.layers = [Layer(ls, self.ctx) for ls in spec.layers]
         if spec.streams and (spec.embed_norm is not None or spec.depth_mix or spec.pass_inputs or spec.embed_additions
                              or spec.embed_position is not None):

@@ -231,9 +231,9 @@ class Attention(Mixer):
         ok = getattr(self.ops, "sink_attention_tiles_ok", None)
         if ok is None or not ok(self.ctx.act_dtype, self.ctx.act_dtype, self.hd, self.vd):
             return None
-        # a causal mask, a window or runs, with or without a sink, run on the kernel of the plain form
+        # a causal mask, a window or runs, with or without a sink, run on the kernel of the plain form where it takes the pages
         plain = not (self.keep_first or self.pool or self.weights_rule == "sigmoid")
-        return self.NEEDS if plain else self.NEEDS_GENERAL
+        return self.NEEDS if plain and self.ops.prefill_pages_ok(self.ctx.page_size) else self.NEEDS_GENERAL
 
     def plan_step(self, step, captured):
         """How the key ranges of a batch of decoded tokens are cut.  Requests of about the same length share one

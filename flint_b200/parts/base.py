@@ -111,6 +111,7 @@ class BuildContext:
     compute: str                   # "bfloat16" or "float32"
     shared: dict = field(default_factory=dict)   # things built once per model (position tables)
     max_context: int | None = None               # positions the model is built to serve (None: the architecture's limit)
+    page_size: int = 64                          # positions a page of the cache holds
 
     @property
     def act_dtype(self):

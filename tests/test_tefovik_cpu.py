@@ -54,6 +54,20 @@ def compare(out, steps, plain, tol=3e-4):
         assert err < tol * max(1.0, float(want.abs().max())), f"step {k}: max error {err:.2e}"
 
 
+@pytest.mark.parametrize("page,rows", [(64, 128), (16, 128), (8, 128), (128, 128), (4, 64), (48, 64), (96, 64)])
+def test_layers_ask_for_tiles_that_the_kernel_for_their_pages_takes(page, rows):
+    """Runs and windows go to the tcgen05 kernel in tiles of 128 rows where it takes the pages, else to the kernel of 64."""
+    from flint_b200.csrc.ops import CudaOps
+    from flint_b200.parts.attention import Attention
+    from flint_b200.parts.base import BuildContext
+    ops = type("Ops", (), {n: staticmethod(getattr(CudaOps, n)) for n in ("sink_attention_tiles_ok", "prefill_pages_ok")})()
+    params = {"hidden_size": 64, "num_heads": 2, "num_kv_heads": 1, "head_dim": 32, "chunk": 9, "position": None}
+    part = Attention(params, BuildContext(ops, torch.device("cpu"), "bfloat16", page_size=page))
+    assert part.step_needs().tile_rows == rows
+    pooled = Attention({**params, "chunk": 0, "window": 64, "pool": 8}, BuildContext(ops, torch.device("cpu"), "bfloat16", page_size=page))
+    assert pooled.step_needs().tile_rows == 64
+
+
 def test_the_plain_mechanisms_hold_their_invariants():
     # the convolution's last column weighs the current token, and nothing comes from before the sequence
     u = torch.arange(1.0, 6.0, dtype=F64)[:, None]
