@@ -97,6 +97,7 @@ class StepStaging:
         smallest = min((n.tile_min_rows for n in self.needs), default=8)
         self.max_tiles = self.max_tokens // max(smallest, 1) + 16
         self._extra = None          # pinned and device buffers of the further tilings, made at first use
+        self._all_rows = None       # the rows of a step that no further tiling takes
         n = 6 * self.max_tokens + 4 * self.max_tiles
         self.host = torch.zeros(n, dtype=torch.int32)
         if self.device.type == "cuda":
@@ -157,6 +158,11 @@ class StepStaging:
         """A further tiling (a model whose mixers declare different needs), cut on the host and uploaded with a
         copy of its own."""
         M, per = self.max_tokens, self.max_tokens + 4 * self.max_tiles
+        if all(len(e.tokens) < needs.tile_min_rows for e in entries):       # decoded tokens: nothing to cut or upload
+            if self._all_rows is None:
+                self._all_rows = torch.arange(M, dtype=torch.int32, device=self.device)
+            T = starts[-1] + len(entries[-1].tokens)
+            return Tiling(self.dev[:0].view(-1, 4), 0, self._all_rows[:T], T, needs.tile_rows)
         if self._extra is None:
             n = per * (len(self.needs) - 1)
             host = torch.zeros(n, dtype=torch.int32)

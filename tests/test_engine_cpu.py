@@ -258,6 +258,20 @@ def test_tiles_of_a_step_come_in_the_order_of_their_last_position():
     assert ends3 == sorted(ends3) and third.other_rows[:third.n_other_rows].tolist() == [20]
 
 
+def test_decoded_tokens_are_not_cut_a_second_time():
+    """A model whose mixers declare two tilings: a batch without a long portion uploads nothing for the second."""
+    from flint_b200.engine.step import StepEntry, StepNeeds, StepStaging
+    needs = (StepNeeds(16, 4), StepNeeds(8, 3))
+    st = StepStaging(96, "cpu", needs=needs)
+    ctx = st.pack([StepEntry(3, 9, [1]), StepEntry(1, 0, [2, 3]), StepEntry(0, 4, [5])], 10, 100)
+    for n in needs:
+        t = ctx.tiling(n)
+        assert (t.n_tiles, t.n_other_rows, t.other_rows.tolist(), t.tile_rows) == (0, 4, [0, 1, 2, 3], n.tile_rows)
+    assert st._extra is None
+    t = st.pack([StepEntry(3, 9, [1]), StepEntry(1, 0, [2, 3, 4])], 10, 100).tiling(needs[1])
+    assert (t.n_tiles, t.other_rows.tolist(), t.tiles.tolist()) == (1, [0], [[1, 3, 1, 0]])
+
+
 def test_decode_attention_is_cut_into_splits_that_cover_the_keys():
     """The plan of the decode attention: the splits cover every key, and with more than four of them they come
     in fours (the four warps of a block then hold one row's splits and merge them themselves)."""
