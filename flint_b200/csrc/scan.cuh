@@ -322,13 +322,14 @@ token_scan_kernel(const ScanArgs a) {
 template <int LANES, int NR, int CPT, int RULE, bool VEC, bool TRANSPOSED>
 inline cudaError_t launch_one(const ScanArgs& a, int n_seq, int threads, cudaStream_t stream) {
   auto kernel = token_scan_kernel<LANES, NR, CPT, RULE, VEC, TRANSPOSED>;
-  static const cudaError_t raised =
-      cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           SCAN_STAGES * TB * scan_token_floats<LANES, NR, CPT, RULE>(256) * (int)sizeof(float));
-  if (raised != cudaSuccess) return raised;
   const int cols = threads / LANES * CPT;
   const dim3 grid((unsigned)((a.V + cols - 1) / cols), (unsigned)a.H, (unsigned)n_seq), block((unsigned)threads);
   const size_t smem = (size_t)SCAN_STAGES * TB * scan_token_floats<LANES, NR, CPT, RULE>(threads) * sizeof(float);
+  if (smem > 48 * 1024) {        // at every launch, and always the same: the limit is one of the call's device
+    const cudaError_t raised = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                    SCAN_STAGES * TB * scan_token_floats<LANES, NR, CPT, RULE>(256) * (int)sizeof(float));
+    if (raised != cudaSuccess) return raised;
+  }
   // An ordinary launch, on an empty chip, where the few blocks get an SM each: started early they land beside the blocks
   // of the kernel before, several to an SM (a prompt of 2,048 tokens then ran half a millisecond longer a layer).
   cudaLaunchConfig_t cfg = {};
