@@ -219,7 +219,7 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
       mbar_expect_tx(bar, values ? v_bytes : k_bytes);
       const uint32_t dst = kv_smem + s * kv_stage_bytes + (values ? k_bytes : 0);
       const int kv0 = (tile_lo + i) * BKV;
-      if (!bt) {                // row of the batch that holds key kv0; rows behind the request's last are masked
+      if (!bt) {                // row of the batch that holds key kv0; rows behind the request's last are masked, their values zeroed
         const int row = row0 - pos0 + kv0;
         if (values) {
           for (int c = 0; c < v_chunks; ++c) tma_load_2d(dst + c * BKV * 128, &map_v, kvh * p.v_step + c * 64, row, bar);
@@ -234,7 +234,7 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
         const int key = kv0 + pc * piece;
         const int lp = key / P;
         int page = lp < p.max_pages ? bt[lp] : -1;
-        if (page < 0) page = 0;   // never visible to these queries (masked): any finite page will do
+        if (page < 0) page = 0;   // never visible to these queries (masked, its values zeroed): any page will do
         const int row = (page * p.nkv + kvh) * P + key % P;
         for (int c = 0; c < (values ? v_chunks : chunks); ++c)
           tma_load_2d(dst + c * BKV * 128 + pc * piece * 128, values ? &map_v : &map_k, c * 64, row, bar);
@@ -376,6 +376,21 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
         if (!ok) break;
       }
       l += (s4[0] + s4[1]) + (s4[2] + s4[3]);
+      // Keys of the tile that none of its rows sees (behind the last, before the first) may be another request's, or what a
+      // page holds from an earlier one.  Their probability is zero, but zero times an infinity is not: their values become zeros.
+      const int unseen_lo = k_lo - kv0, unseen_hi = k_hi - kv0;
+      if (unseen_lo > 0 || unseen_hi < BKV) {
+        const int s = i % STAGES;
+        ok = wait(bar_vfull0 + 8 * s, (i / STAGES) & 1);
+        if (!ok) break;
+        const uint32_t v_src = kv_smem + s * kv_stage_bytes + k_bytes;
+        for (int u = r; u < BKV * 8; u += BQ) {         // 16 bytes of a key's row; the swizzle stays within the row
+          if ((u >> 3) >= unseen_lo && (u >> 3) < unseen_hi) continue;
+          for (int c = 0; c < v_chunks; ++c)
+            asm volatile("st.shared.v4.b32 [%0], {%1, %1, %1, %1};" ::"r"(v_src + c * BKV * 128 + u * 16), "r"(0) : "memory");
+        }
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+      }
       // hand P (and the rescaled O) to the tensor core (the barrier counts all 128 rows; no thread waits on
       // another here)
       tc_fence_before();

@@ -163,6 +163,24 @@ def test_attention_over_the_batch_s_own_rows(ops, H, D, V, C, window, sinks):
     assert (got - want).abs().max() < 4e-2
 
 
+@pytest.mark.parametrize("window", [0, 50])
+@pytest.mark.parametrize("bad", [float("inf"), float("nan")])
+def test_own_rows_beside_rows_that_are_no_numbers(ops, bad, window):
+    """A request whose rows hold infinities changes no bit of its neighbours', before and behind it in the batch."""
+    H, D, R, V, C, lens = 2, 64, 64, 48, 64, (100, 90, 130)
+    T, g = sum(lens), torch.Generator().manual_seed(window)
+    bf = lambda *shape: torch.randn(*shape, generator=g).bfloat16().to(DEV)
+    q_plain, qa, kv, rows = bf(T, H, D), bf(T, H, C + R), bf(T, H * (D + V)), bf(T, C + R)
+    tiles = torch.tensor([[r0 + r, min(128, n - r), slot, r] for slot, (r0, n) in enumerate(((0, 100), (100, 90), (190, 130)))
+                          for r in range(0, n, 128)], dtype=torch.int32, device=DEV)
+    out = [torch.zeros(T, H, V, dtype=torch.bfloat16, device=DEV) for _ in range(2)]
+    for o in out:
+        ops.attention_own_rows(q_plain, qa, C, kv, rows, C, tiles, len(tiles), o, H, D, R, V, window, (D + R) ** -0.5)
+        kv[100:190], rows[100:190] = bad, bad
+    assert torch.isfinite(out[0]).all()
+    assert torch.equal(out[0][:100], out[1][:100]) and torch.equal(out[0][190:], out[1][190:])
+
+
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 def test_latent_attention_window_edges(ops, dtype):
     """With a window the key just inside is seen and the key just outside is not (the mixer's window is a

@@ -176,6 +176,37 @@ def test_masks_in_tiles_of_128_rows(ops, H, G, d, dv, window, chunk, sinks):
         assert (out.float() - want.float()).abs().max().item() < 4e-2
 
 
+@pytest.mark.parametrize("window,chunk,sinks", [(0, 0, True), (0, 40, False), (70, 0, True), (70, 0, False)])
+@pytest.mark.parametrize("P_", [16, 64])
+@pytest.mark.parametrize("bad", [float("inf"), float("nan")])
+def test_masked_tiles_beside_pages_that_hold_no_numbers(ops, P_, bad, window, chunk, sinks):
+    """What pages hold behind a request's last position, and in place of pages that a window gave back, changes no bit."""
+    from flint_b200.engine.step import Tiling
+    g = torch.Generator().manual_seed(window + chunk)
+    H, G, d, dv, n = 4, 2, 64, 48, 203
+    rn = lambda *s: torch.randn(*s, generator=g, dtype=F64)
+    view, _ = paged_kv([rn(n, G, d), rn(30, G, d)], [rn(n, G, dv), rn(30, G, dv)], P_, torch.bfloat16, seed=2)
+    q = torch.randn(43, H * d, generator=g).to(torch.bfloat16).to(DEV)
+    sink = torch.randn(H, generator=g).to(DEV) if sinks else None
+    i32 = lambda x: torch.tensor(x, dtype=torch.int32, device=DEV)
+    tiling = Tiling(i32([[0, 43, 0, 160]]), 1, i32([]), 0, 128)
+    out = [torch.zeros(43, H * dv, dtype=torch.bfloat16, device=DEV) for _ in range(2)]
+    table = view.block_table[0].tolist()
+    for o in out:
+        ops.sink_attention(q, view, step_of(list(range(160, n)), [0] * 43, 1), o, H, G, d, dv, window, 0, sink, d ** -0.5, tiling=tiling, chunk=chunk)
+        for cache in (view.k, view.v):
+            first = 160 - window + 1 if window else 160 if chunk else 0          # the first position that any row sees
+            held = {table[p // P_] for p in range(first, n)}
+            for page in range(cache.shape[0]):
+                if page not in held:
+                    cache[page] = bad
+            cache[table[first // P_], :, :first % P_] = bad
+            cache[table[(n - 1) // P_], :, (n - 1) % P_ + 1:] = bad
+        view.block_table[0, :first // P_] = -1
+    assert torch.isfinite(out[0]).all() and torch.equal(out[0], out[1])
+    assert int(ops.tc_error.item()) == 0
+
+
 def batches_of(pieces, starts, slots_of):
     """pieces: list of batches, a batch a list of (request, first token, count) -> per batch (rows of the flat
     arrays, positions, slots, where each request's rows start, whether every request brings one token)."""
