@@ -49,7 +49,8 @@ class LatentAttention(Mixer):
 
     graph_safe = True
     returns_pending = True
-    # portions of at least 16 rows that start at position 0 attend with the keys and values made, in tiles of 128 rows
+    # portions of at least 16 rows attend with the keys and values made, in tiles of 128 rows, where all of a step start at
+    # position 0 (in layers without a query latent and sinks)
     NEEDS = StepNeeds(tile_rows=128, tile_min_rows=16)
 
     def __init__(self, params, ctx):
@@ -131,22 +132,22 @@ class LatentAttention(Mixer):
     def step_needs(self):
         D, R, V = self.D, self.R, self.V
         ok = (hasattr(self.ops, "attention_own_rows") and self.ctx.act_dtype == torch.bfloat16 and D in (64, 128) and R == 64
-              and 16 <= V <= 128 and V % 16 == 0 and self.C % 8 == 0)
+              and 16 <= V <= 128 and V % 16 == 0 and self.C % 8 == 0 and not self.q_rank and not self.sinks)
         return self.NEEDS if ok else None
 
     def _own_rows(self, step, cache):
         """The tiles of the step's rows that see the step's own rows only, or None.  There the keys and values are worth
         making: 2,048 tokens of 16 heads cost 4 C (D + V) = 0.5 M multiply-adds a token and head, and attention over them
         (D + R + V) a pair of tokens where attention over the latents costs 2 C + R, 3.4 times as many.  Rows of a portion
-        that starts later see rows of earlier steps, and keep to the latents."""
-        if self.w_ukv is None or self.q_rank or self.w_sink is not None or step.n_tokens == len(step.entries) or cache.k.dtype != torch.bfloat16:
+        that starts later see rows of earlier steps, and keep to the latents; so do layers with a query latent or sinks."""
+        if self.w_ukv is None or step.n_tokens == len(step.entries) or cache.k.dtype != torch.bfloat16:
             return None
         tiling = step.tiling(self.NEEDS)
         if not tiling.n_tiles or any(e.start_pos for e in step.entries if len(e.tokens) >= self.NEEDS.tile_min_rows):
             return None
         return tiling
 
-    def _attend_own_rows(self, tiling, q_plain, qa, cache, step, gate):
+    def _attend_own_rows(self, tiling, q_plain, qa, cache, step):
         ops, H, D, R, V, C = self.ops, self.H, self.D, self.R, self.V, self.C
         T, dev = q_plain.shape[0], q_plain.device
         rows = torch.empty((T, self.row_w), dtype=torch.bfloat16, device=dev)
@@ -154,19 +155,14 @@ class LatentAttention(Mixer):
         kv = torch.empty((T, H * (D + V)), dtype=torch.bfloat16, device=dev)
         ops.gemm(rows[:, :C], self.w_ukv, kv)
         attn = torch.empty((T, H, V), dtype=torch.bfloat16, device=dev)
-        ops.attention_own_rows(q_plain, qa, C, kv, rows, C, tiling.tiles, tiling.n_tiles, attn, H, D, R, V, self.window, self.scale,
-                               self.w_sink)
+        ops.attention_own_rows(q_plain, qa, C, kv, rows, C, tiling.tiles, tiling.n_tiles, attn, H, D, R, V, self.window, self.scale)
         if tiling.n_other_rows:            # decoded tokens and short portions beside them: over the latents
             at = tiling.other_rows.long()
             single = all(len(e.tokens) == 1 for e in step.entries if len(e.tokens) < self.NEEDS.tile_min_rows)
             few = SimpleNamespace(pos=step.pos[at], slot=step.slot[at], max_kv_len=step.max_kv_len,
                                   entries=(None,) * tiling.n_other_rows if single else ())
             attn.index_copy_(0, at, self._attend_latents(q_plain[at], qa[at], cache, few, None))
-        if gate is None:
-            return attn
-        out = torch.empty_like(attn)
-        ops.head_finish(attn.view(T, H * V), step.pos, None, None, "half", gate, out.view(T, H * V), H, V)
-        return out
+        return attn
 
     def _attend_latents(self, q_plain, qa, cache, step, gate):
         ops, H, V, C = self.ops, self.H, self.V, self.C
@@ -217,7 +213,7 @@ class LatentAttention(Mixer):
         ops.latent_prepare(q_proj, step.pos, step.slot, self.cos, self.sin, self.rot, self.rot_style, self.w_norm, self.eps,
                            q_plain, qa, cache, H, D, R, C, writes_cache, step.status)
         own = self._own_rows(step, cache)
-        attn = self._attend_own_rows(own, q_plain, qa, cache, step, gate) if own is not None else \
+        attn = self._attend_own_rows(own, q_plain, qa, cache, step) if own is not None else \
             self._attend_latents(q_plain, qa, cache, step, gate)
         # the output projection is handed on as partial sums
         return Pending(partials=ops.gemm_partials(attn.view(T, H * V), self.w_o))

@@ -484,6 +484,50 @@ def test_replay_matches_plain_under_every_cut(setup, dtype):
             assert max(max(g.pages.pool.served) for g in rp.model.cache.groups) >= 2
 
 
+def test_latent_rows(ops):
+    """The cached rows of a batch's tokens, zeros where a position has no page."""
+    C, R, P_ = 40, 8, 16
+    view, dense = paged_rows([torch.randn(n, C + R, generator=torch.Generator().manual_seed(n)) for n in (37, 5)], C + R, P_, torch.bfloat16)
+    view.block_table[0, 1] = -1
+    pos, slot = list(range(37)) + [4, 0, 300], [0] * 37 + [1, 1, 1]
+    out = torch.full((40, C + R), 7.0, dtype=torch.bfloat16, device=DEV)
+    i32 = lambda x: torch.tensor(x, dtype=torch.int32, device=DEV)
+    ops.latent_rows(view, i32(pos), i32(slot), out)
+    want = torch.cat([dense[0][:, :C + R], dense[1][[4, 0], :C + R], torch.zeros(1, C + R, dtype=torch.float64)])
+    want[16:32] = 0.0
+    assert torch.equal(out.cpu().double(), want)
+
+
+def test_whole_prompts_with_keys_and_values_made(tmp_path, monkeypatch):
+    """Whole prompts of several tiles alone and together, beside decoded tokens and short portions, and beside a later portion
+    (when all keep to the latents), against the plain model.  Bound: as under every cut in bfloat16."""
+    from flint_b200.parts.latent_attention import LatentAttention
+    cfg, lens = tiny.P3, (150, 40, 333, 130, 70)
+    folder, w = tiny.write_model(tmp_path / "m", cfg, seed=3)
+    reqs = traces.make_requests(cfg["vocab"], lens, seed=7)
+    made = []
+    attend = LatentAttention._attend_own_rows
+    monkeypatch.setattr(LatentAttention, "_attend_own_rows", lambda self, tiling, *a: made.append(tiling.n_tiles) or attend(self, tiling, *a))
+    part = lambda rid, lo, hi: {"id": rid, "tokens": reqs[rid][lo:hi], "want": list(range(hi - lo))}
+    batches = [([part("r0", 0, 146)], 2),                                                          # one prompt, two tiles
+               ([part("r1", 0, 12), part("r0", 146, 147)], 0),                                     # short and decoded
+               ([part("r0", 147, 148), part("r2", 0, 300), part("r1", 12, 15), part("r3", 0, 128)], 4),
+               ([part("r0", 148, 149), part("r3", 128, 129), part("r4", 0, 65)], 1),               # beside decoded tokens only
+               ([part("r2", 300, 333), part("r0", 149, 150), part("r1", 15, 20)], 0),              # a later portion
+               ([part("r1", 20, 40), part("r4", 65, 70), part("r3", 129, 130)], 0)]
+    steps = [{"step": i, "entries": e, "end": []} for i, (e, _) in enumerate(batches)]
+    for page_size in (64, 16):
+        made.clear()
+        rp = Replayer(folder, dtype="bfloat16", max_tokens=1024, page_size=page_size, max_requests=5, device=DEV)
+        out = {s["step"]: rp.run_step(s["entries"]) for s in steps}
+        assert made == [n for _, n in batches for _ in cfg["layers"] if n]
+        exp = traces.expected_rows(steps, {rid: P.forward(cfg, w, t) for rid, t in reqs.items()})
+        assert set(out) == set(exp)
+        errs = torch.cat([rel_err(out[k], torch.stack(rows)) for k, rows in exp.items()])
+        bad = int((errs > 4e-2).sum())
+        assert bad <= 0.02 * len(errs), f"{bad} of {len(errs)} rows, worst {float(errs.max()):.3g}"
+
+
 def test_long_decoding_token_by_token(setup):
     """Two requests decoded side by side, one token a step each, over several pages, after prompts of unequal
     length: the captured decode step is replayed hundreds of times."""

@@ -54,6 +54,19 @@ P2 = {
     ],
 }
 
+# P3: 64 plain and 64 rotated dims, as whole prompts need that attend with the keys and values made, a layer that reads
+# another's latent, no feed-forwards (nothing is chosen, so that every row of every cut can be compared).  Not among
+# CONFIGS: its own test runs it.
+P3 = {
+    "architecture": "Puledra", "vocab": 96, "width": 128, "norm": {"eps": 1e-6},
+    "embedding": {"scale": 1.0},
+    "layers": [
+        _layer(_mixer(3, 64, 64, 64, 16, 64, 10000.0), None),
+        _layer(_mixer(2, 64, 64, 64, 48, 64, 10000.0, kv_from=0), None),
+        _layer(_mixer(2, 128, 64, 64, 128, 72, 500000.0), None),
+    ],
+}
+
 CONFIGS = {"P1": P1, "P2": P2}
 
 
