@@ -450,7 +450,7 @@ __device__ __forceinline__ void arrive_in_cluster(uint32_t bar) {
 }
 
 template <bool GATED, bool RELU2>
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS)
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1)
 gemm_tc_wide_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x, const WideParams p,
                     const GateParams gp) {
   extern __shared__ uint8_t smem_raw[];
@@ -498,7 +498,10 @@ gemm_tc_wide_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
     return false;
   };
 
+  // Dependents start when every block runs; those that take tensor memory find no room in shared memory beside one.  Over
+  // experts only after the wait, see flint_gemm_tc.
   if (map_pending) pdl_wait();
+  pdl_launch();
   const int tiles_n = grouped ? *p.n_tiles : (p.rows + p.row_step - 1) / p.row_step;
   const int n_items = tiles_m * tiles_n * p.splits;
 
@@ -528,34 +531,39 @@ gemm_tc_wide_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
   };
 
   const uint32_t leader_full = place_in(full0, 0), leader_acc_empty = place_in(acc_empty0, 0);
+  // a CTA's rows of a tile come in boxes of x_box
+  auto boxes_of = [&](const Item& w) { return ((w.mma_n >> 1) + p.x_box - 1) / p.x_box; };
+  const uint32_t box_bytes = p.x_box * BK * 2;
+  auto expect = [&](int boxes, int s) {              // what both CTAs bring
+    if (rank == 0) mbar_expect_tx(full0 + 8 * s, 2 * (A_BYTES + boxes * box_bytes));
+  };
   auto load_w = [&](const Item& w, int s, int i) {
     tma_load_2d_pair(tiles + s * STAGE_BYTES, &map_w, (w.kb0 + i) * BK, w.w_row, leader_full + 8 * s);
   };
-  auto load_x = [&](const Item& w, int s, int i) {
-    const int half = w.mma_n >> 1;
-    for (int b = 0; b * p.x_box < half; ++b)
-      tma_load_2d_pair(tiles + s * STAGE_BYTES + A_BYTES + b * p.x_box * BK * 2, &map_x, (w.kb0 + i) * BK,
-                       w.row0 + rank * half + b * p.x_box, leader_full + 8 * s);
+  auto load_x = [&](const Item& w, int boxes, int s, int i) {
+    const int row = w.row0 + rank * (w.mma_n >> 1);
+    for (int b = 0; b < boxes; ++b)
+      tma_load_2d_pair(tiles + s * STAGE_BYTES + A_BYTES + b * box_bytes, &map_x, (w.kb0 + i) * BK, row + b * p.x_box,
+                       leader_full + 8 * s);
   };
-  auto expect = [&](const Item& w, int s) {          // what both CTAs bring
-    if (rank == 0) mbar_expect_tx(full0 + 8 * s, 2 * (A_BYTES + ((w.mma_n >> 1) + p.x_box - 1) / p.x_box * p.x_box * BK * 2));
-  };
-  // the weights of the first ring do not depend on the kernel before this one
+  // the weights of the first ring do not depend on the kernel before this one, its rows do
   int ahead = 0;
   if (warp == 0 && lane == 0) {
     Item w;
     if (item_at(pair, w)) {
+      const int boxes = boxes_of(w);
       ahead = w.nkb < WIDE_STAGES ? w.nkb : WIDE_STAGES;
       for (int i = 0; i < ahead; ++i) {
-        expect(w, i);
+        expect(boxes, i);
         load_w(w, i, i);
       }
+      pdl_wait();
+      for (int i = 0; i < ahead; ++i) load_x(w, boxes, i, i);
     }
   }
-  // Tensor memory is taken by a pair that has met, when every earlier kernel has ended, and dependents start only when every
-  // pair has its own: no wait for tensor memory (it has no limit) can then stand against another kernel's.  Taken at the top,
-  // by each CTA before it knew of the other and beside earlier kernels' blocks, prompts of 470 rows and more through four
-  // layers of width 2,048 did not end.
+  // Tensor memory is taken by a pair that has met, when every earlier kernel has ended: no wait for it (it has no limit) can
+  // then stand against another kernel's.  Taken at the top, by each CTA before it knew of the other and beside earlier
+  // kernels' blocks, prompts of 470 rows and more through four layers of width 2,048 did not end.
   pdl_wait();
   __syncwarp();
   if (warp == 1) {
@@ -567,25 +575,22 @@ gemm_tc_wide_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
   cluster_sync();
   tc_fence_after();
   const uint32_t tmem = tmem_holder;
-  pdl_launch();
 
   if (given_up) {
     // nothing to do but to leave
   } else if (warp == 0 && lane == 0) {
     // ---------------------------------------------------------------- TMA producer of this CTA's halves
-    int kc = 0;
+    int kc = ahead;
     bool ok = true;
     Item w;
     for (int it = pair; ok && item_at(it, w); it += pairs) {
-      int i = 0;
-      for (; i < ahead; ++i, ++kc) load_x(w, i, i);
-      ahead = 0;
-      for (; i < w.nkb; ++i, ++kc) {
+      const int boxes = boxes_of(w);
+      for (int i = it == pair ? ahead : 0; i < w.nkb; ++i, ++kc) {
         const int s = kc % WIDE_STAGES;
         if (!wait(empty0 + 8 * s, ((kc / WIDE_STAGES) & 1) ^ 1)) { ok = false; break; }
-        expect(w, s);
+        expect(boxes, s);
         load_w(w, s, i);
-        load_x(w, s, i);
+        load_x(w, boxes, s, i);
       }
     }
   } else if (warp == 1 && lane == 0 && rank == 0) {
