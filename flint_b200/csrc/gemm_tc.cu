@@ -384,8 +384,9 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
 // products, and each CTA's tensor memory receives its own 128 features of all the tile's tokens, so the epilogue is that of
 // one CTA's tile.  What bounds it: an SM takes in about 64 bytes a cycle from L2, and a CTA alone with 128 x 256 tiles needs
 // 48 KB a K block (measured at that limit: 117 GB/s an SM, 410 ns a K block), a CTA of the pair 32 KB for as many products:
-// 378 to 424 ns, where the library product of 8,192^3 that gives the burst peak works out at 377.  3,500 rows: N 16,384 K 4,096
-// 445 -> 349 us (1,350 TFLOP/s), N 4,096 K 16,384 422 -> 372; 2,048 rows, N 6,144 K 4,096 98 -> 82 us.
+// 378 to 424 ns, where the library product of 8,192^3 that gives the burst peak works out at 377.  Weights from HBM, a CTA alone
+// and pairs in turn on one chip: 3,500 rows, N 16,384 K 4,096 454 -> 342 us (1,374 TFLOP/s), N 4,096 K 16,384 572 -> 436; 2,048
+// rows, N 6,144 K 4,096 120 -> 95, N = 4,096 78 -> 69; 900 rows, N 4,096 K 2,048 35 -> 27.
 // Tiles go out in bands of WIDE_BAND row tiles, rows first: the tiles that run at the same time then share few weight
 // rows and few token rows (feature tiles first, a 134 MB weight was read again for every row tile).
 constexpr int WIDE_ROWS = 256;       // most token rows of a tile
