@@ -298,8 +298,9 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
       const Item w = item_at(j);
       if (!w.valid) break;
       const int buf = j & 1;
-      // every lane goes on or none does: what follows is the whole warp's
-      if (!__all_sync(0xffffffffu, mbar_wait(acc_full0 + 8 * buf, (j >> 1) & 1, ab, p.wait_cycles))) break;
+      // Where the wait ran out, for some lanes or all, every lane goes on: what follows is the whole warp's, and what it leaves
+      // is not used (the flag is up).  A vote here cost 1 % of a decode step at batch 1.
+      mbar_wait(acc_full0 + 8 * buf, (j >> 1) & 1, ab, p.wait_cycles);
       tc_fence_after();
       if (!waited) { pdl_wait(); waited = true; }   // before reading or writing what earlier kernels touch
       // output feature of this thread: its lane of the accumulator, or, gated, one of the warp's 16
