@@ -253,36 +253,33 @@ constexpr int SEG = RPT + 4;     // floats between the rows of neighbouring lane
 // TPC: threads per column (D <= 32 TPC).  RULE: the state-space form (one decay per head, plain write) or the gated delta
 // rule (the write corrected by what the state already returns for the key) with a decay per key channel or per head.
 // q, k [T, G D] and v [T, H V] are float32 views with row strides; decay [T, H D] (DELTA_CHANNEL) or [T, H]; w1 [T, H]: dt
-// (STATE_SPACE) or beta; skip [H] or null.  seq_start [n_seq + 1] or null (row e is request e).  Grid: (column blocks, H, n_seq).
+// (STATE_SPACE) or beta; skip [H] or null.  Row t is request t's token.  Grid: (column blocks, H, T).
 // VEC: every row of q, k, v and decay starts on a 16-byte boundary and D and V are multiples of 4, so the operands are
 // staged 16 bytes a copy; else 4 bytes a copy.  Both leave the same numbers in the same places.
+template <int TPC, int RULE>
+__host__ __device__ constexpr int token_floats() {      // q, k (and the decay per channel), the block's values, and two numbers
+  return (RULE == DELTA_CHANNEL ? 3 : 2) * TPC * SEG + SCAN_THREADS / TPC + 4;
+}
+
 template <int TPC, int RULE, bool VEC>
 __global__ void __launch_bounds__(SCAN_THREADS)
-recurrence_scan_kernel(const float* __restrict__ q, long long q_stride, const float* __restrict__ k, long long k_stride,
-                       const float* __restrict__ v, long long v_stride, const float* __restrict__ decay,
-                       const float* __restrict__ w1, const float* __restrict__ skip, const int* __restrict__ slot,
-                       const int* __restrict__ seq_start, float* __restrict__ state, long long state_stride,
-                       float* __restrict__ o, int H, int G, int D, int V, int TB) {
-  extern __shared__ __align__(16) float sm[];
+recurrence_token_kernel(const float* __restrict__ q, long long q_stride, const float* __restrict__ k, long long k_stride,
+                        const float* __restrict__ v, long long v_stride, const float* __restrict__ decay,
+                        const float* __restrict__ w1, const float* __restrict__ skip, const int* __restrict__ slot,
+                        float* __restrict__ state, long long state_stride, float* __restrict__ o, int H, int G, int D, int V) {
   constexpr int DP = TPC * SEG;                  // floats of a staged vector of key dims: lane s of a column reads from s SEG
   constexpr bool CHANNEL = RULE == DELTA_CHANNEL;
-  constexpr int NV = CHANNEL ? 3 : 2;            // staged vectors a token: q, k (and the decay per channel)
+  constexpr int NV = CHANNEL ? 3 : 2;            // staged vectors: q, k (and the decay per channel)
   constexpr int COLS = SCAN_THREADS / TPC;       // columns a block takes
+  __shared__ __align__(16) float tok[token_floats<TPC, RULE>()];
   const int tid = threadIdx.x, sub = tid % TPC, col = blockIdx.x * COLS + tid / TPC;
-  const int h = blockIdx.y, e = blockIdx.z, kh = h / (H / G);
-  const int r0 = seq_start ? seq_start[e] : e, r1 = seq_start ? seq_start[e + 1] : e + 1;
-  if (r1 <= r0) return;
-  // a stage: TB tokens of q, k (and decay per channel), the columns' values, and two numbers a token
-  const int per_tok = NV * DP + COLS + 4;        // a multiple of 4: the operands are read as float4
-  float* stage[2] = {sm, sm + (size_t)TB * per_tok};
-  for (int i = tid; i < 2 * TB * per_tok; i += SCAN_THREADS) {      // dims beyond D: q = k = 0, decay = 1
-    const int w = i % per_tok;
-    sm[i] = (CHANNEL && w >= 2 * DP && w < 3 * DP) ? 1.f : 0.f;
-  }
+  const int h = blockIdx.y, t = blockIdx.z, kh = h / (H / G);
+  for (int i = tid; i < token_floats<TPC, RULE>(); i += SCAN_THREADS)      // dims beyond D: q = k = 0, decay = 1
+    tok[i] = (CHANNEL && i >= 2 * DP && i < 3 * DP) ? 1.f : 0.f;
   __syncthreads();
   pdl_wait();
   const bool live = col < V;
-  float* S_g = state + (size_t)slot[r0] * state_stride + (size_t)h * D * V;
+  float* S_g = state + (size_t)slot[t] * state_stride + (size_t)h * D * V;
   float S[RPT];
 #pragma unroll
   for (int i = 0; i < RPT; ++i) {
@@ -290,109 +287,81 @@ recurrence_scan_kernel(const float* __restrict__ q, long long q_stride, const fl
     S[i] = (live && d < D) ? S_g[(size_t)d * V + col] : 0.f;
   }
   const int c0 = blockIdx.x * COLS, nc = min(COLS, V - c0);
-  const float* q_h = q + (size_t)kh * D;
-  const float* k_h = k + (size_t)kh * D;
-  const float* g_h = CHANNEL ? decay + (size_t)h * D : nullptr;
-  const float* v_h = v + (size_t)h * V + c0;
-  auto fetch = [&](int t0, int st) {
-    const int n = min(TB, r1 - t0);
-    float* base = stage[st];
-    if (VEC) {
-      // piece j of a token: 16 bytes of q, then of k, then of the decay, then of the values
-      const int d4 = D >> 2, pieces = NV * d4 + (nc >> 2);
-      for (int j = tid; j < pieces; j += SCAN_THREADS) {
-        int a = 0, x = j;                        // which vector, which piece of it
-        if (x >= d4) { x -= d4; a = 1; }
-        if (a == 1 && x >= d4) { x -= d4; a = 2; }
-        if (CHANNEL && a == 2 && x >= d4) { x -= d4; a = 3; }
-        const bool val = a == NV;
-        const int d = 4 * x;
-        const int off = val ? NV * DP + d : a * DP + (d / RPT) * SEG + d % RPT;
-        const float* src = val ? v_h + d : (a == 0 ? q_h : a == 1 ? k_h : g_h) + d;
-        const long long stride = val ? v_stride : a == 0 ? q_stride : a == 1 ? k_stride : (long long)H * D;
-        for (int tt = 0; tt < n; ++tt) copy16(base + (size_t)tt * per_tok + off, src + (size_t)(t0 + tt) * stride);
-      }
-    } else {
-      for (int i = tid; i < n * D; i += SCAN_THREADS) {
-        const int tt = i / D, d = i % D, t = t0 + tt;
-        float* dst = base + (size_t)tt * per_tok + (d / RPT) * SEG + d % RPT;
-        copy4(dst, q_h + (size_t)t * q_stride + d);
-        copy4(dst + DP, k_h + (size_t)t * k_stride + d);
-        if (CHANNEL) copy4(dst + 2 * DP, g_h + (size_t)t * H * D + d);
-      }
-      for (int i = tid; i < n * nc; i += SCAN_THREADS) {
-        const int tt = i / nc, c = i % nc;
-        copy4(base + (size_t)tt * per_tok + NV * DP + c, v_h + (size_t)(t0 + tt) * v_stride + c);
-      }
+  const float* q_h = q + (size_t)t * q_stride + (size_t)kh * D;
+  const float* k_h = k + (size_t)t * k_stride + (size_t)kh * D;
+  const float* g_h = CHANNEL ? decay + ((size_t)t * H + h) * D : nullptr;
+  const float* v_h = v + (size_t)t * v_stride + (size_t)h * V + c0;
+  if (VEC) {
+    // piece j: 16 bytes of q, then of k, then of the decay, then of the values
+    const int d4 = D >> 2, pieces = NV * d4 + (nc >> 2);
+    for (int j = tid; j < pieces; j += SCAN_THREADS) {
+      int a = 0, x = j;                        // which vector, which piece of it
+      if (x >= d4) { x -= d4; a = 1; }
+      if (a == 1 && x >= d4) { x -= d4; a = 2; }
+      if (CHANNEL && a == 2 && x >= d4) { x -= d4; a = 3; }
+      const int d = 4 * x;
+      if (a == NV) copy16(tok + NV * DP + d, v_h + d);
+      else copy16(tok + a * DP + (d / RPT) * SEG + d % RPT, (a == 0 ? q_h : a == 1 ? k_h : g_h) + d);
     }
-    for (int tt = tid; tt < n; tt += SCAN_THREADS) {
-      float* dst = base + (size_t)tt * per_tok + NV * DP + COLS;
-      copy4(dst, w1 + (size_t)(t0 + tt) * H + h);
-      if (!CHANNEL) copy4(dst + 1, decay + (size_t)(t0 + tt) * H + h);
+  } else {
+    for (int d = tid; d < D; d += SCAN_THREADS) {
+      float* dst = tok + (d / RPT) * SEG + d % RPT;
+      copy4(dst, q_h + d);
+      copy4(dst + DP, k_h + d);
+      if (CHANNEL) copy4(dst + 2 * DP, g_h + d);
     }
-    asm volatile("cp.async.commit_group;" ::: "memory");
-  };
-  const float skip_h = skip ? skip[h] : 0.f;
-  fetch(r0, 0);
-  int st = 0;
-  for (int t0 = r0; t0 < r1; t0 += TB, st ^= 1) {
-    if (t0 + TB < r1) {
-      fetch(t0 + TB, st ^ 1);
-      asm volatile("cp.async.wait_group 1;" ::: "memory");
-    } else {
-      asm volatile("cp.async.wait_group 0;" ::: "memory");
-    }
-    __syncthreads();
-    const int n = min(TB, r1 - t0);
-    for (int tt = 0; tt < n; ++tt) {
-      const float* tok = stage[st] + (size_t)tt * per_tok;
-      const float4* q4 = reinterpret_cast<const float4*>(tok + sub * SEG);
-      const float4* k4 = reinterpret_cast<const float4*>(tok + DP + sub * SEG);
-      const float* rest = tok + NV * DP;
-      const float vj = rest[tid / TPC], w = rest[COLS];
-      float4 kr[RPT / 4];                        // the key's dims of this lane, read once for both passes
-#pragma unroll
-      for (int i = 0; i < RPT / 4; ++i) kr[i] = k4[i];
-      float u;
-      if (RULE != STATE_SPACE) {
-        const float4* g4 = reinterpret_cast<const float4*>(tok + 2 * DP + sub * SEG);
-        const float a = CHANNEL ? 0.f : rest[COLS + 1];
-        float d0 = 0.f, d1 = 0.f, d2 = 0.f, d3 = 0.f;
-#pragma unroll
-        for (int i = 0; i < RPT / 4; ++i) {
-          const float4 gg = CHANNEL ? g4[i] : make_float4(a, a, a, a);
-          S[4 * i] *= gg.x; S[4 * i + 1] *= gg.y; S[4 * i + 2] *= gg.z; S[4 * i + 3] *= gg.w;
-          d0 = fmaf(S[4 * i], kr[i].x, d0); d1 = fmaf(S[4 * i + 1], kr[i].y, d1);
-          d2 = fmaf(S[4 * i + 2], kr[i].z, d2); d3 = fmaf(S[4 * i + 3], kr[i].w, d3);
-        }
-        float dot = (d0 + d1) + (d2 + d3);
-#pragma unroll
-        for (int m = 1; m < TPC; m <<= 1) dot += __shfl_xor_sync(0xffffffffu, dot, m);
-        u = w * (vj - dot);
-      } else {
-        const float a = rest[COLS + 1];
-#pragma unroll
-        for (int i = 0; i < RPT; ++i) S[i] *= a;
-        u = w * vj;
-      }
-      float o0 = 0.f, o1 = 0.f, o2 = 0.f, o3 = 0.f;
-#pragma unroll
-      for (int i = 0; i < RPT / 4; ++i) {
-        const float4 qq = q4[i];
-        S[4 * i] = fmaf(kr[i].x, u, S[4 * i]); S[4 * i + 1] = fmaf(kr[i].y, u, S[4 * i + 1]);
-        S[4 * i + 2] = fmaf(kr[i].z, u, S[4 * i + 2]); S[4 * i + 3] = fmaf(kr[i].w, u, S[4 * i + 3]);
-        o0 = fmaf(S[4 * i], qq.x, o0); o1 = fmaf(S[4 * i + 1], qq.y, o1);
-        o2 = fmaf(S[4 * i + 2], qq.z, o2); o3 = fmaf(S[4 * i + 3], qq.w, o3);
-      }
-      float out = (o0 + o1) + (o2 + o3);
-#pragma unroll
-      for (int m = 1; m < TPC; m <<= 1) out += __shfl_xor_sync(0xffffffffu, out, m);
-      if (live && sub == 0) o[(size_t)(t0 + tt) * H * V + (size_t)h * V + col] = fmaf(skip_h, vj, out);
-    }
-    __syncthreads();          // the stage is refilled in the next round
+    for (int c = tid; c < nc; c += SCAN_THREADS) copy4(tok + NV * DP + c, v_h + c);
   }
-  // Only now may the kernel behind this one start: its blocks would wait on the SMs beside the walk's few warps for
-  // as long as the walk takes (a prompt of 2,048 tokens ran twice as long with the release at the top).
+  if (tid == 0) {
+    copy4(tok + NV * DP + COLS, w1 + (size_t)t * H + h);
+    if (!CHANNEL) copy4(tok + NV * DP + COLS + 1, decay + (size_t)t * H + h);
+  }
+  const float skip_h = skip ? skip[h] : 0.f;
+  asm volatile("cp.async.commit_group;" ::: "memory");
+  asm volatile("cp.async.wait_group 0;" ::: "memory");
+  __syncthreads();
+  const float4* q4 = reinterpret_cast<const float4*>(tok + sub * SEG);
+  const float4* k4 = reinterpret_cast<const float4*>(tok + DP + sub * SEG);
+  const float* rest = tok + NV * DP;
+  const float vj = rest[tid / TPC], w = rest[COLS];
+  float4 kr[RPT / 4];                        // the key's dims of this lane, read once for both passes
+#pragma unroll
+  for (int i = 0; i < RPT / 4; ++i) kr[i] = k4[i];
+  float u;
+  if (RULE != STATE_SPACE) {
+    const float4* g4 = reinterpret_cast<const float4*>(tok + 2 * DP + sub * SEG);
+    const float a = CHANNEL ? 0.f : rest[COLS + 1];
+    float d0 = 0.f, d1 = 0.f, d2 = 0.f, d3 = 0.f;
+#pragma unroll
+    for (int i = 0; i < RPT / 4; ++i) {
+      const float4 gg = CHANNEL ? g4[i] : make_float4(a, a, a, a);
+      S[4 * i] *= gg.x; S[4 * i + 1] *= gg.y; S[4 * i + 2] *= gg.z; S[4 * i + 3] *= gg.w;
+      d0 = fmaf(S[4 * i], kr[i].x, d0); d1 = fmaf(S[4 * i + 1], kr[i].y, d1);
+      d2 = fmaf(S[4 * i + 2], kr[i].z, d2); d3 = fmaf(S[4 * i + 3], kr[i].w, d3);
+    }
+    float dot = (d0 + d1) + (d2 + d3);
+#pragma unroll
+    for (int m = 1; m < TPC; m <<= 1) dot += __shfl_xor_sync(0xffffffffu, dot, m);
+    u = w * (vj - dot);
+  } else {
+    const float a = rest[COLS + 1];
+#pragma unroll
+    for (int i = 0; i < RPT; ++i) S[i] *= a;
+    u = w * vj;
+  }
+  float o0 = 0.f, o1 = 0.f, o2 = 0.f, o3 = 0.f;
+#pragma unroll
+  for (int i = 0; i < RPT / 4; ++i) {
+    const float4 qq = q4[i];
+    S[4 * i] = fmaf(kr[i].x, u, S[4 * i]); S[4 * i + 1] = fmaf(kr[i].y, u, S[4 * i + 1]);
+    S[4 * i + 2] = fmaf(kr[i].z, u, S[4 * i + 2]); S[4 * i + 3] = fmaf(kr[i].w, u, S[4 * i + 3]);
+    o0 = fmaf(S[4 * i], qq.x, o0); o1 = fmaf(S[4 * i + 1], qq.y, o1);
+    o2 = fmaf(S[4 * i + 2], qq.z, o2); o3 = fmaf(S[4 * i + 3], qq.w, o3);
+  }
+  float out = (o0 + o1) + (o2 + o3);
+#pragma unroll
+  for (int m = 1; m < TPC; m <<= 1) out += __shfl_xor_sync(0xffffffffu, out, m);
+  if (live && sub == 0) o[((size_t)t * H + h) * V + col] = fmaf(skip_h, vj, out);
   pdl_launch();
 #pragma unroll
   for (int i = 0; i < RPT; ++i) {
@@ -1088,14 +1057,11 @@ extern "C" int flint_recurrence_scan(const float* q, long long q_stride, const f
     if (rc != cudaSuccess) return fail("recurrence_scan: %s", cudaGetErrorString(rc));
     return check_launch("recurrence_scan");
   }
-  const int tpc = D <= 32 ? 1 : D <= 64 ? 2 : D <= 128 ? 4 : 8;
-  const int dp = tpc * SEG, cols = SCAN_THREADS / tpc;
-  const int tb = tpc <= 2 ? 16 : tpc <= 4 ? 8 : 4;
-  const size_t smem = (size_t)2 * tb * ((rule == DELTA_CHANNEL ? 3 : 2) * dp + cols + 4) * sizeof(float);
+  const int tpc = D <= 32 ? 1 : D <= 64 ? 2 : D <= 128 ? 4 : 8, cols = SCAN_THREADS / tpc;
   const dim3 grid((unsigned)((V + cols - 1) / cols), (unsigned)H, (unsigned)n_seq), block(SCAN_THREADS);
 #define SCAN(TPC, RULE, VEC)                                                                                           \
-  launch_pdl(recurrence_scan_kernel<TPC, RULE, VEC>, grid, block, smem, stream, q, q_stride, k, k_stride, v,   \
-              v_stride, decay, w1, skip, slot, seq_start, state, state_stride, o, H, G, D, V, tb)
+  launch_pdl(recurrence_token_kernel<TPC, RULE, VEC>, grid, block, 0, stream, q, q_stride, k, k_stride, v, v_stride,   \
+             decay, w1, skip, slot, state, state_stride, o, H, G, D, V)
 #define SCAN_T(TPC)                                                                                       \
   do {                                                                                                    \
     if (rule == DELTA_CHANNEL) { if (vec) SCAN(TPC, DELTA_CHANNEL, true); else SCAN(TPC, DELTA_CHANNEL, false); } \

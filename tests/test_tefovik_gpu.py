@@ -406,6 +406,27 @@ def test_walk_over_many_columns(ops, rule, H, G, D, V):
     assert (state.cpu().double().view(n + 1, H, D, V) - final).abs().max() < 2e-5 * float(final.abs().max())
 
 
+@pytest.mark.parametrize("rule", ["state_space", "delta", "delta_head"])
+@pytest.mark.parametrize("H,G,D,V", [(32, 8, 128, 128), (64, 8, 128, 64), (16, 16, 256, 64), (6, 3, 60, 33)])
+def test_a_decoded_token_is_the_walk_s_to_rounding(ops, rule, H, G, D, V):
+    """Single tokens take another kernel than the rows of a prompt: sums in another order.  Bound: sums of D float32 products."""
+    g = torch.Generator().manual_seed(H + D + V)
+    n, delta, channel = 9, rule != "state_space", rule == "delta"
+    q, k = torch.randn(n, G * D, generator=g) * D ** -0.5, torch.nn.functional.normalize(torch.randn(n, G, D, generator=g), dim=-1).view(n, G * D)
+    v, skip = torch.randn(n, H * V, generator=g), torch.randn(H, generator=g).to(DEV)
+    decay, w = torch.rand(n, H * D if channel else H, generator=g).to(DEV), torch.rand(n, H, generator=g).to(DEV)
+    start = torch.randn(n, H * D * V, generator=g)
+    slot = torch.arange(n - 1, -1, -1, dtype=torch.int32, device=DEV)
+    got = []
+    for seq in (None, torch.arange(n + 1, dtype=torch.int32, device=DEV)):
+        state, out = start.to(DEV), torch.zeros(n, H * V, device=DEV)
+        ops.recurrence_scan(q.to(DEV), k.to(DEV), v.to(DEV), decay, delta, w if delta else None, None if delta else w,
+                            None if delta else skip, slot, seq, n, state, out, H, G, D, V)
+        got.append((out, state))
+    for a, b in zip(*got):
+        assert (a - b).abs().max() < D * 2 ** -23 * float(b.abs().max())
+
+
 def tables(pos_max, dims, base):
     half = max(dims // 2, 1)
     ang = torch.arange(pos_max + 1, dtype=F64)[:, None] * base ** (-2.0 * torch.arange(half, dtype=F64) / max(dims, 1))[None, :]
