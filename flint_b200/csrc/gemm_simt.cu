@@ -234,7 +234,7 @@ extern "C" int flint_gemm_simt(const void* x, int x_dtype, int ldx, const void* 
   // that can be read in whole pieces of four
   const int x_size = x_dtype == FLINT_F32 ? 4 : 2, w_size = w_dtype == FLINT_F32 ? 4 : 2;
   const long long large = (long long)((M + WM - 1) / WM) * ((N + WN - 1) / WN);
-  if (!tile_expert && !gated && large >= 148 && K % 4 == 0 && ldx % 4 == 0 && (uintptr_t)x % (4 * x_size) == 0 &&
+  if (!tile_expert && !gated && large >= multiprocessors() && K % 4 == 0 && ldx % 4 == 0 && (uintptr_t)x % (4 * x_size) == 0 &&
       (uintptr_t)w % (4 * w_size) == 0) {
     const dim3 wide((N + WN - 1) / WN, (M + WM - 1) / WM);
     FLINT_DISPATCH_DTYPE(x_dtype, TX, FLINT_DISPATCH_DTYPE(w_dtype, TW, FLINT_DISPATCH_DTYPE(out_dtype, TO,

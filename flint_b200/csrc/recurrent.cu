@@ -1162,7 +1162,7 @@ extern "C" int flint_branch_mean(int n, const float* const* partials, const long
   for (int b = 0; b < n; ++b)
     lined = lined && strides[b] % 4 == 0 && !(((uintptr_t)partials[b] | (uintptr_t)bias[b] | (uintptr_t)w[b]) & 15);
   // few rows want all their loads in flight at once: a wide block a row
-  if (T >= 148 && lined && n <= 2 && W <= 4 * 4 * ROW_THREADS) {
+  if (T >= multiprocessors() && lined && n <= 2 && W <= 4 * 4 * ROW_THREADS) {
     if (W <= 2 * 4 * ROW_THREADS) launch_pdl(branch_mean_rows_kernel<2>, dim3((unsigned)T), dim3(ROW_THREADS), 0, stream, bl, eps, out, W);
     else launch_pdl(branch_mean_rows_kernel<4>, dim3((unsigned)T), dim3(ROW_THREADS), 0, stream, bl, eps, out, W);
     return check_launch("branch_mean");
@@ -1178,7 +1178,7 @@ extern "C" int flint_post_norm(float* x, const float* partials, int n_partials, 
   if (n_partials < 1) return fail("post_norm: needs at least one partial sum");
   const bool lined = W % 4 == 0 && partial_stride % 4 == 0 &&
                      !(((uintptr_t)x | (uintptr_t)partials | (uintptr_t)bias | (uintptr_t)s | (uintptr_t)gamma | (uintptr_t)beta | (uintptr_t)copy) & 15);
-  if (T >= 148 && lined && W <= 4 * 4 * ROW_THREADS) {          // few rows: a wide block a row, as below
+  if (T >= multiprocessors() && lined && W <= 4 * 4 * ROW_THREADS) {          // few rows: a wide block a row, as below
 #define POST_ROWS(V)                                                                                                         \
   FLINT_DISPATCH_DTYPE(copy_dtype, TC,                                                                                       \
       (launch_pdl(post_norm_rows_kernel<V, TC>, dim3((unsigned)T), dim3(ROW_THREADS), 0, stream, x, partials, n_partials,    \

@@ -986,7 +986,7 @@ int row_norm_form(const RowArgs& a, int rows, const RowPlan& p, cudaStream_t str
     constexpr int ROWS = 4;
     const int n_warps = ROWS * p.threads / 32, groups = (a.E + 3) / 4, k = n_warps >= groups ? n_warps / groups : 1;
     const size_t smem = (size_t)ROWS * (a.H + a.E * k) * sizeof(float);
-    if (a.wr && p.cl == 1 && rows >= ROWS * 148 && p.threads <= 128 && a.H % 8 == 0 && !((uintptr_t)a.wr & 15) && smem <= 110 * 1024) {
+    if (a.wr && p.cl == 1 && rows >= ROWS * multiprocessors() && p.threads <= 128 && a.H % 8 == 0 && !((uintptr_t)a.wr & 15) && smem <= 110 * 1024) {
       static bool wide_configured = false;
       return launch_row(row_norm_kernel<VPT, TW, ST, ROWS>, wide_configured, a, (rows + ROWS - 1) / ROWS, ROWS * p.threads, smem, stream);
     }

@@ -349,13 +349,7 @@ inline cudaError_t launch_one(const ScanArgs& a, int n_seq, int threads, cudaStr
 // one column 1,130; 16 heads, 1,024 tokens: 277 against 213).
 template <int RULE, bool TRANSPOSED>
 inline cudaError_t launch_token_scan(const ScanArgs& a, int n_seq, bool vec, cudaStream_t stream) {
-  static int sm_count = 0;
-  if (!sm_count) {
-    int dev = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sm_count, cudaDevAttrMultiProcessorCount, dev);
-    if (sm_count <= 0) sm_count = 148;
-  }
+  const int sm_count = flint::multiprocessors();
   const long long columns = (long long)n_seq * a.H * a.V;
 #define SCAN_ONE(L, NR, C)                                                              \
   return vec ? launch_one<L, NR, C, RULE, true, TRANSPOSED>(a, n_seq, threads, stream) \
